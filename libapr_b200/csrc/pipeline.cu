@@ -1887,16 +1887,18 @@ int work_pitch(int yn, int xn, int zn) {
 }
 
 // The y pass into padded lines: the input is padded and smoothed about 2^26
-// samples at a time, so the copy stays small.
+// samples at a time, so the copy takes the volume's padded size and at most 134
+// MB (138 MB on the longest rows).
 static void launch_smooth_y_padded(const uint16_t *img, float *work, int yn, int pitch, uint64_t nlines, float lambda,
                                    unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s) {
     APRB_PROF("bspline_y", s);
     const IIRDev c = dev_coef(iir_coefficients(lambda, yn));
-    uint64_t step = std::max<uint64_t>(1024, (uint64_t(1) << 26) / (uint64_t)pitch);
+    const uint64_t step = std::max<uint64_t>(1024, (uint64_t(1) << 26) / (uint64_t)pitch);
+    const uint64_t most = std::min(step + 31, nlines);  // lines of the longest run
     for (uint64_t l0 = 0; l0 < nlines;) {
         uint64_t n = std::min(step, nlines - l0);
         if (nlines - l0 - n < 32) n = nlines - l0;  // no run of fewer lines than a CTA's
-        uint16_t *buf = img_pad.as_on<uint16_t>((step + 32) * (uint64_t)pitch, s);
+        uint16_t *buf = img_pad.as_on<uint16_t>(most * (uint64_t)pitch, s);
         pad_lines_kernel<<<blocks_for(n * (uint64_t)(pitch / 8), 256), 256, 0, s>>>(img + l0 * (uint64_t)yn, yn, pitch,
                                                                                   n, buf);
         count_launch();
