@@ -479,8 +479,7 @@ PixelOut<IT> pixel_stages(aprb_converter *c, const aprb_params &p, const uint16_
     unsigned *mm = c->mm.as_on<unsigned>(2, s);
     float *d_off = c->offset.as_on<float>(1, s);
     unsigned *d_err = c->err.as_on<unsigned>(2, s);  // [0] overflow count, [1] TMA wait timeout
-    const int pitch = !is_u16 && !host && p.lambda > 0 ? work_pitch(yn, xn, zn) : yn;
-    c->pitch = pitch;
+    int pitch = !is_u16 && !host && p.lambda > 0 ? work_pitch(yn, xn, zn) : yn;
     IT *work = c->work.as_on<IT>((uint64_t)pitch * xn * zn, s);
     if (host) {
         launch_upload_smooth<IT>(host, const_cast<uint16_t *>(img), work, yn, xn, zn, p.lambda, mm, d_off,
@@ -491,8 +490,9 @@ PixelOut<IT> pixel_stages(aprb_converter *c, const aprb_params &p, const uint16_
         }
     } else {
         launch_minmax_offset(img, n, mm, d_off, is_u16 && p.lambda > 0, s);
-        launch_smooth<IT>(img, work, yn, xn, zn, pitch, p.lambda, d_off, d_err, c->iir_ckpt, c->img_pad, s);
+        pitch = launch_smooth<IT>(img, work, yn, xn, zn, pitch, p.lambda, d_off, d_err, c->iir_ckpt, c->img_pad, s);
     }
+    c->pitch = pitch;
     IT *grad = c->grad.as_on<IT>(nd, s);
     float *ids_raw = c->ids_raw.as_on<float>(nd, s);
     float *ids = c->ids.as_on<float>(nd, s);

@@ -78,11 +78,12 @@ void launch_minmax_offset(const uint16_t *img, uint64_t n, unsigned *mm, float *
 // Elements between the lines of the float working image of a device volume: y_num,
 // or padded to a multiple of 8 where that lets the vector and TMA kernels run.
 int work_pitch(int yn, int xn, int zn);
-// work: lines `pitch` elements apart; padded lines (pitch != yn, float only)
-// are packed through img_pad
+// work: room for lines `pitch` elements apart; padded lines (pitch != yn, float
+// only) are packed through img_pad.  Returns the pitch that work has: yn where
+// the TMA pass that padded lines need is not to be had.
 template <typename IT>
-void launch_smooth(const uint16_t *img, IT *work, int yn, int xn, int zn, int pitch, float lambda,
-                   const float *d_offset, unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s);
+int launch_smooth(const uint16_t *img, IT *work, int yn, int xn, int zn, int pitch, float lambda,
+                  const float *d_offset, unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s);
 template <typename IT>
 void launch_upload_smooth(const uint16_t *host, uint16_t *img, IT *work, int yn, int xn, int zn, float lambda,
                           unsigned *mm, float *d_offset, int apply, unsigned *d_err, DevBuf &ckpt,

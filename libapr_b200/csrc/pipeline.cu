@@ -1888,8 +1888,9 @@ int work_pitch(int yn, int xn, int zn) {
 
 // The y pass into padded lines: the input is padded and smoothed about 2^26
 // samples at a time, so the copy takes the volume's padded size and at most 134
-// MB (138 MB on the longest rows).
-static void launch_smooth_y_padded(const uint16_t *img, float *work, int yn, int pitch, uint64_t nlines, float lambda,
+// MB (138 MB on the longest rows).  False when the TMA pass does not take a run
+// (no tensor maps from this driver); nothing of work is then of use.
+static bool launch_smooth_y_padded(const uint16_t *img, float *work, int yn, int pitch, uint64_t nlines, float lambda,
                                    unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s) {
     APRB_PROF("bspline_y", s);
     const IIRDev c = dev_coef(iir_coefficients(lambda, yn));
@@ -1905,27 +1906,27 @@ static void launch_smooth_y_padded(const uint16_t *img, float *work, int yn, int
         APRB_CHECK_LAUNCH();
         const uint64_t nck = n * (uint64_t)((yn + kAY - 1) / kAY);
         if (!launch_iir_y_tma(buf, work + l0 * (uint64_t)pitch, yn, pitch, n, c, d_err + 1, ckpt.as_on<float2>(nck, s),
-                              nck, s)) {
-            set_error("the padded y pass does not take this layout");
-            throw Error{APRB_ERR_CUDA};
-        }
+                              nck, s))
+            return false;
         l0 += n;
     }
+    return true;
 }
 
 template <typename IT>
-void launch_smooth(const uint16_t *img, IT *work, int yn, int xn, int zn, int pitch, float lambda,
-                   const float *d_offset, unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s) {
+int launch_smooth(const uint16_t *img, IT *work, int yn, int xn, int zn, int pitch, float lambda,
+                  const float *d_offset, unsigned *d_err, DevBuf &ckpt, DevBuf &img_pad, cudaStream_t s) {
     if constexpr (std::is_same<IT, float>::value) {
-        if (pitch != yn) {
-            launch_smooth_y_padded(img, work, yn, pitch, (uint64_t)xn * zn, lambda, d_err, ckpt, img_pad, s);
+        if (pitch != yn &&
+            launch_smooth_y_padded(img, work, yn, pitch, (uint64_t)xn * zn, lambda, d_err, ckpt, img_pad, s)) {
             launch_smooth_x<IT>(work, pitch, xn, zn, lambda, d_err, ckpt, s);
             launch_smooth_z<IT>(work, pitch, xn, zn, lambda, d_err, ckpt, s);
-            return;
+            return pitch;
         }
     }
     launch_smooth_yx<IT>(img, work, yn, xn, zn, lambda, d_offset, d_err, ckpt, s);
     launch_smooth_z<IT>(work, yn, xn, zn, lambda, d_err, ckpt, s);
+    return yn;
 }
 
 // Offset and smoothing of a volume that is still in host memory: it is copied
@@ -2263,10 +2264,10 @@ template void launch_upload_smooth<uint16_t>(const uint16_t *, uint16_t *, uint1
                                              cudaStream_t);
 template void launch_upload_smooth<float>(const uint16_t *, uint16_t *, float *, int, int, int, float, unsigned *,
                                           float *, int, unsigned *, DevBuf &, cudaStream_t, cudaStream_t);
-template void launch_smooth<uint16_t>(const uint16_t *, uint16_t *, int, int, int, int, float, const float *, unsigned *,
-                                      DevBuf &, DevBuf &, cudaStream_t);
-template void launch_smooth<float>(const uint16_t *, float *, int, int, int, int, float, const float *, unsigned *,
-                                   DevBuf &, DevBuf &, cudaStream_t);
+template int launch_smooth<uint16_t>(const uint16_t *, uint16_t *, int, int, int, int, float, const float *, unsigned *,
+                                     DevBuf &, DevBuf &, cudaStream_t);
+template int launch_smooth<float>(const uint16_t *, float *, int, int, int, int, float, const float *, unsigned *,
+                                  DevBuf &, DevBuf &, cudaStream_t);
 template void launch_gradient<uint16_t>(const uint16_t *, int, int, int, int, uint16_t *, float *, float *, int, int, int,
                                         const aprb_params &, unsigned *, cudaStream_t);
 template void launch_gradient<float>(const float *, int, int, int, int, float *, float *, float *, int, int, int,

@@ -46,8 +46,30 @@ static long check_copy(int yn, uint64_t nlines) {
     return bad;
 }
 
+// launch_smooth: padded lines where every run is taken, else the passes of
+// unpadded lines over the whole volume, and the pitch that the image then has
+static long check_fallback() {
+    DevBuf ckpt, pad;
+    std::vector<float> origin(1);
+    std::vector<uint16_t> img(1);
+    g_work = origin.data();
+    g_pad = &pad;
+    long bad = 0;
+    for (int accept : {0, 1, 2, 1 << 30}) {
+        g_accept = accept;
+        g_passes.clear();
+        const int pitch = launch_smooth<float>(img.data(), g_work, 517, 400, 400, 520, 3.0f, nullptr, nullptr, ckpt,
+                                               pad, nullptr);
+        const bool padded = accept >= 2;  // two runs
+        bad += pitch != (padded ? 520 : 517) || g_passes != (padded ? "x520 z520 " : "yx517 z517 ");
+    }
+    if (bad) std::printf("refused layouts: %ld faults\n", bad);
+    return bad;
+}
+
 int main() {
     long bad = 0;
+    bad += check_fallback();
     for (int yn : {65, 66, 67, 129, 517, 1013, 4095, 65534}) {
         const uint64_t step = std::max<uint64_t>(1024, (uint64_t(1) << 26) / ((yn + 7) & ~7));
         // the smallest volume that is padded, whole runs, and rests of 1 .. 33 lines

@@ -1,8 +1,9 @@
 """The padded y pass of the smoothing (rows of 4k + 1 .. 4k + 3 samples),
-checked on the CPU: launch_smooth_y_padded and its copy kernel are taken
-verbatim from libapr_b200/csrc/pipeline.cu and compiled with g++ behind the
-stand-ins of tests/cpp/padded_prelude.hpp; tests/cpp/padded_main.cpp looks at
-the runs it makes, at the size of the padded copy and at the copy."""
+checked on the CPU: launch_smooth, launch_smooth_y_padded and its copy kernel
+are taken verbatim from libapr_b200/csrc/pipeline.cu and compiled with g++ behind
+the stand-ins of tests/cpp/padded_prelude.hpp; tests/cpp/padded_main.cpp looks at
+the runs it makes, at the size of the padded copy, at the copy and at what
+happens where the TMA pass does not take a run."""
 import os
 import re
 import shutil
@@ -27,7 +28,8 @@ def _function(src, name):
 def _translation_unit():
     with open(os.path.join(ROOT, "libapr_b200", "csrc", "pipeline.cu")) as f:
         src = f.read()
-    body = "".join(_function(src, n) for n in ("void pad_lines_kernel(", "launch_smooth_y_padded(const uint16_t"))
+    body = "".join(_function(src, n) for n in ("void pad_lines_kernel(", "launch_smooth_y_padded(const uint16_t",
+                                                  "launch_smooth(const uint16_t"))
     body, n = re.subn(r"pad_lines_kernel<<<.*?>>>\(", "run_pad(", body, flags=re.S)
     assert n == 1
     with open(os.path.join(CPP, "padded_prelude.hpp")) as f:
