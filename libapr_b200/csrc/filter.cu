@@ -22,10 +22,7 @@
 // (run_convolution_pencil, :706-736).  A cell no particle covers holds a
 // sentinel; reading it is counted as a stale read (the reference would read a
 // stale pencil buffer there) and contributes 0.
-#include <climits>
-
 #include "kernels.cuh"
-#include "tma.cuh"
 
 namespace aprb {
 
@@ -691,13 +688,16 @@ __global__ void __launch_bounds__(kConvThreads<T>, 4) conv_block_kernel(
     if (nstale) atomicAdd(stale, (unsigned long long)nstale);
 }
 
-// Planes of a level image at most: about 1 GiB, so that the scratch of a large
-// level stays a fraction of its particles'; whole tiles.  whole: all planes.
+// Planes of a run: its image, halo planes included, takes at most 1 GiB, so
+// that the scratch of a large level stays a fraction of its particles'; whole
+// tiles, one at least, so levels of more than 2^30 / (kTZ + 2R + 1) bytes a plane
+// (4900^2 floats at 3^3) take kTZ + 2R + 1 planes.  whole: all planes.
 template <int R, typename T>
 int image_run(const LD &d, bool whole) {
-    const ImageShape<R, T> one(d, 0, 1);
-    const uint64_t run = (uint64_t(1) << 30) / (one.plane * sizeof(T)) / kTZ * kTZ;
-    return whole || run >= (uint64_t)d.zn ? d.zn : std::max<int>(kTZ, (int)run);
+    const int64_t halo = 2 * R + 1;
+    const int64_t fit = (int64_t)((uint64_t(1) << 30) / (ImageShape<R, T>(d, 0, 1).plane * sizeof(T))) - halo;
+    if (whole || fit >= d.zn) return d.zn;
+    return (int)std::min<int64_t>(d.zn, std::max<int64_t>(kTZ, fit / kTZ * kTZ));
 }
 
 template <int R, typename T>

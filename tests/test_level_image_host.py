@@ -1,0 +1,63 @@
+"""The runs of planes that a level's neighbourhood image is made in, checked on
+the CPU: ImageShape and image_run are taken verbatim from
+libapr_b200/csrc/filter.cu and compiled with g++.  The image of a run, its halo
+planes included, takes at most 1 GiB, or a tile's eight planes and their halo
+where those are more; runs are whole tiles; in place, one run has all planes."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from tests.conftest import ROOT
+
+MAIN = r"""
+template <int R, typename T>
+static long check(int xn, int yn, int zn) {
+    const LD d{yn, xn, zn};
+    long bad = image_run<R, T>(d, true) != zn;
+    const int run = image_run<R, T>(d, false);
+    bad += run < 1 || run > zn || (run < zn && run % kTZ != 0);
+    const uint64_t bytes = ImageShape<R, T>(d, 0, run).elems() * sizeof(T);
+    const uint64_t least = ImageShape<R, T>(d, 0, std::min(zn, kTZ)).elems() * sizeof(T);
+    bad += bytes > std::max(uint64_t(1) << 30, least);
+    // as many planes as the bound allows
+    if (run < zn)
+        bad += ImageShape<R, T>(d, 0, std::min(zn, run + kTZ)).elems() * sizeof(T) <= (uint64_t(1) << 30);
+    if (bad) std::printf("R %d, %zu bytes: %d x %d x %d, run %d\n", R, sizeof(T), zn, xn, yn, run);
+    return bad;
+}
+
+int main() {
+    long bad = 0;
+    for (int side : {1, 3, 100, 1000, 2048, 2900, 3400, 4096, 5800, 8192, 16384, 65535})
+        for (int yn : {side, side / 2 + 1})
+            for (int zn : {1, 7, 8, 9, 23, 24, 64, 67, 512, 2000, 65535}) {
+                bad += check<1, float>(side, yn, zn) + check<2, float>(side, yn, zn);
+                bad += check<1, double>(side, yn, zn) + check<2, double>(side, yn, zn);
+            }
+    std::printf("faults %ld\n", bad);
+    return bad != 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_image_runs_keep_their_bound(tmp_path):
+    with open(os.path.join(ROOT, "libapr_b200", "csrc", "filter.cu")) as f:
+        src = f.read()
+
+    def block(start, end="\n}\n"):
+        a = src.index(start)
+        return src[a:src.index(end, a) + len(end)]
+
+    body = "".join([block("struct LD {", "};\n"), block("template <int R, typename T>\nstruct ImageShape {", "\n};\n"),
+                    block("constexpr int kTX", "\n"), block("template <int R, typename T>\nint image_run(")])
+    text = ("#include <algorithm>\n#include <cstdint>\n#include <cstdio>\n#define __host__\n#define __device__\n"
+            + body + MAIN)
+    path = tmp_path / "image_run.cpp"
+    path.write_text(text)
+    exe = str(tmp_path / "image_run")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-o", exe, str(path)], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and "faults 0" in r.stdout, r.stdout[-2000:] + r.stderr
