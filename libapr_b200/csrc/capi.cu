@@ -540,12 +540,13 @@ Readback read_back(aprb_converter *c, const uint64_t *count, const float *offset
     return r;
 }
 
-// Bytes to ask the pool for: whole eighths of a power of two (at least 1 MiB).
-// A particle count differs a little from volume to volume; blocks of their
-// exact sizes seldom fit the next one, and the pool then maps memory anew,
-// which stalls a 2048 x 2048 x 512 conversion for 13 to 800 ms now and then.
+// Bytes to ask the pool for: whole eighths of a power of two (the pool's 512-byte
+// granules below 8 KiB), so at most an eighth more than needed.  A particle
+// count differs a little from volume to volume; blocks of their exact sizes
+// seldom fit the next one, and the pool then maps memory anew, which stalls a
+// 2048 x 2048 x 512 conversion for 13 to 800 ms now and then.
 uint64_t pool_size(uint64_t bytes) {
-    uint64_t step = uint64_t(1) << 20;
+    uint64_t step = 512;
     while (step * 16 <= bytes) step *= 2;
     return (bytes + step - 1) / step * step;
 }
