@@ -113,7 +113,8 @@ struct TreeLevelArgs {
     const uint2 *cw, *ctw;  // row words of the children (ctw null: no tree level)
 };
 
-// One warp per parent row, a lane per cell of a parent word.  The parent's word
+// One warp per parent row, or per part of `per` words of one where rows are long
+// and few, a lane per cell of a parent word.  The parent's word
 // gives the node's index, the words of the four child rows each child pair's
 // source and index, so every load of a node's eight children follows from
 // words alone (a row's nodes are neighbours, and so are their children): no
@@ -121,7 +122,8 @@ struct TreeLevelArgs {
 // Bound by latency: the words come to shared memory 32 at a time, so a step
 // waits for its children only.  512 x 2048 x 2048 APR, all levels: 1.8 ms (words
 // read in each step 3.9, one step ahead in registers 3.2, child rows staged in
-// shared memory cell by cell 3.8).
+// shared memory cell by cell 3.8).  65535 cells in one row: 75 us in parts, 349
+// row by row; 9 x 200 x 4100: 75 against 127 us.
 // SUB: the children may be tree nodes too (not on the finest tree level, whose
 // instance keeps half the row pointers).
 template <bool SUB>
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
                                                                                 const uint64_t *__restrict__ xz_end,
                                                                                 const T *__restrict__ parts,
                                                                                 const uint64_t *__restrict__ t_xz_end,
-                                                                                T *tree) {
+                                                                                T *tree, int per) {
     __shared__ TreeWords<SUB> words[8];
     TreeWords<SUB> &sm = words[threadIdx.x >> 5];
     const uint64_t prow = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // z * xt + x
@@ -142,8 +144,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
     const uint64_t pb = t_xz_end[a.t_row_base + prow - 1], pe = t_xz_end[a.t_row_base + prow];
     if (pb == pe) return;
     const int xp = (int)(prow % (uint64_t)a.dt.xn), zp = (int)(prow / (uint64_t)a.dt.xn);
-    const int nwt = nword(a.dt.yn), nw = nword(a.dc.yn);
-    const uint2 *WN = a.tw + prow * nwt;
+    const int first = (int)blockIdx.y * per;  // of the warp's words; counted from there below
+    const int end = min(per, nword(a.dt.yn) - first), nw = nword(a.dc.yn) - 2 * first;
+    const uint2 *WN = a.tw + prow * nword(a.dt.yn) + first;
     const uint2 *W[4], *WT[4];
     const T *own[4], *sub[4];
 #pragma unroll
@@ -153,10 +156,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
         own[q] = sub[q] = nullptr;
         if (cz < a.dc.zn && cx < a.dc.xn) {
             const uint64_t row = (uint64_t)cz * a.dc.xn + cx;
-            W[q] = a.cw + row * nw;
+            W[q] = a.cw + row * nword(a.dc.yn) + 2 * first;
             own[q] = parts + xz_end[a.c_row_base + row - 1];
             if (SUB) {
-                WT[q] = a.ctw + row * nw;
+                WT[q] = a.ctw + row * nword(a.dc.yn) + 2 * first;
                 sub[q] = tree + t_xz_end[a.ct_row_base + row - 1];
             }
         }
@@ -169,10 +172,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
     const T eighth = T(0.125);
     const unsigned bit = 1u << lane, b = 2 * (lane & 15), low = (1u << b) - 1u;
     constexpr int U = SUB ? 1 : 2;
-    for (int c0 = 0; c0 < nwt; c0 += 32) {
+    for (int c0 = 0; c0 < end; c0 += 32) {
         // the words of 32 parent words, and of the two child words under each
         __syncwarp();
-        sm.node[lane] = c0 + lane < nwt ? WN[c0 + lane] : make_uint2(0u, 0u);
+        sm.node[lane] = c0 + lane < end ? WN[c0 + lane] : make_uint2(0u, 0u);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -183,7 +186,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
                 if (SUB) sm.ws[SUB ? q : 0][SUB ? k : 0] = in ? WT[q][j] : make_uint2(0u, 0u);
             }
         __syncwarp();
-        for (int j0 = 0; j0 < 32 && c0 + j0 < nwt; j0 += U) {
+        for (int j0 = 0; j0 < 32 && c0 + j0 < end; j0 += U) {
             uint2 node[U];
             T v[U][8], vs[U][8];
             unsigned has[U], hast[U];
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) tree_mean_kernel(
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (!(node[u].x & bit)) continue;
-                const T s = T((32 * (c0 + j0 + u) + lane == a.dt.yn - 1) ? syxz : sxz);
+                const T s = T((32 * (first + c0 + j0 + u) + lane == a.dt.yn - 1) ? syxz : sxz);
                 T acc = T(0);
                 // particles first, then tree nodes, each in z, x, y order
 #pragma unroll
@@ -904,6 +907,16 @@ void build_filter_index(const Geom &g, const uint64_t *xz_end, const uint16_t *y
     fi.built = true;
 }
 
+// What a warp takes of `rows` rows of n units: the whole row, or halves of it
+// (whole steps, down to one) while there are fewer than `warps` warps, the SMs'
+// fill.  A row is a serial walk, so on few long rows its length is the kernel's
+// time.
+static int row_part(uint64_t rows, int n, int step, uint64_t warps) {
+    int per = (n + step - 1) / step;
+    while (per > 1 && rows * (uint64_t)((n + per * step - 1) / (per * step)) < warps) per = (per + 1) / 2;
+    return per * step;
+}
+
 // Tree means of every tree level, fine to coarse.
 template <typename T>
 static void tree_means_all(const Geom &g, const uint64_t *xz_end, const Geom &tg, const uint64_t *t_xz_end,
@@ -925,10 +938,12 @@ static void tree_means_all(const Geom &g, const uint64_t *xz_end, const Geom &tg
         ta.ctw = (l <= tg.l_max) ? words + fi.tree_woff[l] : nullptr;
         const uint64_t rows = (uint64_t)ta.dt.xn * ta.dt.zn;
         if (rows == 0) continue;
+        const int nwt = nword(ta.dt.yn), per = row_part(rows, nwt, 2, 148 * 32);
+        const dim3 grid(blocks_for(rows * 32, 256), (unsigned)((nwt + per - 1) / per));
         if (ta.ctw)
-            tree_mean_kernel<true, T><<<blocks_for(rows * 32, 256), 256, 0, s>>>(ta, xz_end, in, t_xz_end, tree);
+            tree_mean_kernel<true, T><<<grid, 256, 0, s>>>(ta, xz_end, in, t_xz_end, tree, per);
         else
-            tree_mean_kernel<false, T><<<blocks_for(rows * 32, 256), 256, 0, s>>>(ta, xz_end, in, t_xz_end, tree);
+            tree_mean_kernel<false, T><<<grid, 256, 0, s>>>(ta, xz_end, in, t_xz_end, tree, per);
         count_launch();
     }
     APRB_CHECK_LAUNCH();

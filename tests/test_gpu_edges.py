@@ -48,8 +48,9 @@ def crossed(shape, seed):
     return img.clip(0, 65535).astype(np.uint16)
 
 
-# levels of 2049, 2113 and of 4161 and 2081 cells along y
-@pytest.mark.parametrize("shape", [(3, 5, 2049), (4, 6, 2113), (2, 3, 4161)])
+# levels of 2049, 2113, of 4161 and 2081 and of 9001 - 2251 cells along y; few rows,
+# so a row also goes to several warps
+@pytest.mark.parametrize("shape", [(3, 5, 2049), (4, 6, 2113), (2, 3, 4161), (1, 1, 9001)])
 def test_filters_on_rows_of_several_parts(shape):
     img, acc, apr = built(shape, 0, img=crossed(shape, 11))
     tree = B.orc_tree(acc)
