@@ -938,7 +938,10 @@ static void tree_means_all(const Geom &g, const uint64_t *xz_end, const Geom &tg
         ta.ctw = (l <= tg.l_max) ? words + fi.tree_woff[l] : nullptr;
         const uint64_t rows = (uint64_t)ta.dt.xn * ta.dt.zn;
         if (rows == 0) continue;
-        const int nwt = nword(ta.dt.yn), per = row_part(rows, nwt, 2, 148 * 32);
+        // eight warps an SM: with 32, the 4096 rows of 4 words of a 128 x 512 x 512 APR
+        // are halved too, and a part's staging costs more than its walk (10 iterations
+        // of Richardson-Lucy 8.71 against 8.55 ms)
+        const int nwt = nword(ta.dt.yn), per = row_part(rows, nwt, 2, 148 * 8);
         const dim3 grid(blocks_for(rows * 32, 256), (unsigned)((nwt + per - 1) / per));
         if (ta.ctw)
             tree_mean_kernel<true, T><<<grid, 256, 0, s>>>(ta, xz_end, in, t_xz_end, tree, per);
