@@ -306,8 +306,8 @@ __device__ __forceinline__ const T *no_cell(bool zero) {
         return reinterpret_cast<const T *>(g_cell_f64) + zero;
 }
 
-// The level image: one warp per row, a lane per pair of cells (2j, 2j + 1),
-// which share their parent.  The row words say which source holds a cell
+// The level image: one warp per row (PARTS: per part of `per` cells, where rows
+// are long and few), a lane per pair of cells (2j, 2j + 1), which share their parent.  The row words say which source holds a cell
 // (particle, parent, tree mean) and at which index, so every cell is one load
 // and one store, with no prefill and no y coordinates read.  Rows that no
 // particle of the level is within R of are not written (nothing reads them).
@@ -315,12 +315,12 @@ __device__ __forceinline__ const T *no_cell(bool zero) {
 // 2048 APR.  The words of 2048 cells come to shared memory at once, so a step
 // waits for its values only (words read in each step: 4.6 ms; one step ahead in
 // registers: 5.2; a word of 32 cells a step instead of 64 in pairs: 5.6).
-template <int R, typename T>
+template <int R, typename T, bool PARTS>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kernel(ConvLevelArgs a, ImageShape<R, T> m,
                                                           const uint64_t *__restrict__ xz_end,
                                                           const T *__restrict__ in,
                                                           const uint64_t *__restrict__ t_xz_end,
-                                                          const T *__restrict__ tree, T *__restrict__ D) {
+                                                          const T *__restrict__ tree, T *__restrict__ D, int per) {
     __shared__ uint2 sm[8][160];
     const int lane = threadIdx.x & 31;
     const unsigned nb = (unsigned)(m.xp + 7) / 8, ip = blockIdx.x / nb;  // plane of the image
@@ -342,9 +342,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
     T *row = D + (uint64_t)ip * m.plane + (uint64_t)pr * m.pitch + m.PADY;
     const int zs = src_index(z, zn, a.reflect), xs = src_index(x, xn, a.reflect);
     const bool row_in = zs >= 0 && xs >= 0;
+    const int first = PARTS ? (int)blockIdx.y * per : 0, end = PARTS ? min(first + per, yn) : yn;  // the warp's cells
     const T none = (a.reflect || (z >= 0 && z < zn && x >= 0 && x < xn)) ? VT<T>::miss() : T(0);
     if (!row_in) {
-        for (int y = lane - R; y < yn + R; y += 32) row[y] = none;
+        for (int y = first + lane - R; y < end + R; y += 32) row[y] = none;
         return;
     }
     const int nw = nword(yn), nwp = nword(a.dp.yn);
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
     constexpr int U = 4;  // steps of 64 cells with their loads in flight
     const uint2 zero = make_uint2(0u, 0u);
     uint2 *sw = sm[threadIdx.x >> 5], *swp = sw + 64, *swt = sw + 96;  // a row's words: own, parents, tree
-    for (int c0 = 0; c0 < yn; c0 += 2048) {
+    for (int c0 = first; c0 < end; c0 += 2048) {
         __syncwarp();
 #pragma unroll
         for (int k = lane; k < 64; k += 32) {
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
         }
         swp[lane] = WP && c0 / 64 + lane < nwp ? WP[c0 / 64 + lane] : zero;
         __syncwarp();
-        for (int y0 = c0; y0 < min(c0 + 2048, yn); y0 += 64 * U) {
+        for (int y0 = c0; y0 < min(c0 + 2048, end); y0 += 64 * U) {
             uint2 w[U], wp[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
             }
         }
     }
-    if (lane < 2 * R) {
+    if (first == 0 && lane < 2 * R) {
         // the R cells before and after the row
         const int y = lane < R ? -1 - lane : yn + lane - R;
         const int ys = src_index(y, yn, a.reflect);
@@ -703,13 +704,29 @@ int image_run(const LD &d, bool whole) {
     return (int)std::min<int64_t>(d.zn, std::max<int64_t>(kTZ, fit / kTZ * kTZ));
 }
 
+// What a warp takes of `rows` rows of n units: the whole row, or halves of it
+// (whole steps, down to one) while there are fewer than `warps` warps, the SMs'
+// fill.  A row is a serial walk, so on few long rows its length is the kernel's
+// time.
+int row_part(uint64_t rows, int n, int step, uint64_t warps) {
+    int per = (n + step - 1) / step;
+    while (per > 1 && rows * (uint64_t)((n + per * step - 1) / (per * step)) < warps) per = (per + 1) / 2;
+    return per * step;
+}
+
 template <int R, typename T>
 T *launch_level_image(const ConvLevelArgs &a, const ImageShape<R, T> &m, const uint64_t *xz_end, const T *in,
                       const uint64_t *t_xz_end, const T *tree, FilterBuffers &fb, cudaStream_t s) {
     APRB_PROF("level_image", s);
     T *D = (T *)fb.dense.get(m.elems() * sizeof(T));
-    const unsigned blocks = (unsigned)((m.xp + 7) / 8) * (unsigned)m.planes();
-    level_image_kernel<R, T><<<blocks, 256, 0, s>>>(a, m, xz_end, in, t_xz_end, tree, D);
+    // whole steps of 256 cells, as many warps as the SMs hold: 3^3 on one row of
+    // 65535 cells 474 -> 250 us
+    const int per = row_part((uint64_t)m.xp * m.planes(), m.yn, 256, 148 * 40);
+    const dim3 grid((unsigned)((m.xp + 7) / 8) * (unsigned)m.planes(), (unsigned)((m.yn + per - 1) / per));
+    if (grid.y > 1)
+        level_image_kernel<R, T, true><<<grid, 256, 0, s>>>(a, m, xz_end, in, t_xz_end, tree, D, per);
+    else
+        level_image_kernel<R, T, false><<<grid, 256, 0, s>>>(a, m, xz_end, in, t_xz_end, tree, D, per);
     count_launch();
     APRB_CHECK_LAUNCH();
     return D;
@@ -905,16 +922,6 @@ void build_filter_index(const Geom &g, const uint64_t *xz_end, const uint16_t *y
     APRB_CUDA(cudaStreamSynchronize(s));
     for (int l = 0; l < 32; ++l) fi.level_count[l] = l < g.l_min || l > g.l_max ? 0 : ends[l + 1] - ends[l];
     fi.built = true;
-}
-
-// What a warp takes of `rows` rows of n units: the whole row, or halves of it
-// (whole steps, down to one) while there are fewer than `warps` warps, the SMs'
-// fill.  A row is a serial walk, so on few long rows its length is the kernel's
-// time.
-static int row_part(uint64_t rows, int n, int step, uint64_t warps) {
-    int per = (n + step - 1) / step;
-    while (per > 1 && rows * (uint64_t)((n + per * step - 1) / (per * step)) < warps) per = (per + 1) / 2;
-    return per * step;
 }
 
 // Tree means of every tree level, fine to coarse.
