@@ -251,9 +251,10 @@ struct ConvLevelArgs {
 // ---------------------------------------------------------------------------
 // Level image of a run of planes [z0, z1): planes z0 - R .. z1 + R, rows
 // -R .. xn + R and cells -R .. yn + R with the boundary folded in -- a cell
-// outside the level holds the value of its reflection (the sentinel when the
-// reflection leaves the level too), or 0 with the zero pad -- so the sums need
-// no boundary case.  Cell y of a row sits at index y + PADY; pitch and PADY
+// outside the level holds the value of its reflection, or 0 with the zero pad
+// and where the reflection leaves the level too (an axis of one cell, or of two at
+// R = 2; such taps are stale reads, and outside_taps counts them) -- so the sums
+// need no boundary case.  Cell y of a row sits at index y + PADY; pitch and PADY
 // keep the pair (2j - R, 2j - R + 1) aligned.  One plane, row and cell more
 // than the taps of the last cell need: an odd extent's last block reads them.
 template <int R, typename T>
@@ -277,7 +278,7 @@ constexpr int kTY = 128;           // cells of its rows
 
 // source index of index i of an axis of length n: i itself, its reflection
 // about the edge sample, or -1 (zero pad, or a reflection that leaves the axis)
-__device__ __forceinline__ int src_index(int i, int n, int reflect) {
+__host__ __device__ __forceinline__ int src_index(int i, int n, int reflect) {
     if (i >= 0 && i < n) return i;
     if (!reflect) return -1;
     const int r = i < 0 ? -i : 2 * (n - 1) - i;
@@ -295,15 +296,15 @@ struct Pair2<double> {
     using type = double2;
 };
 
-// What an uncovered cell copies: the sentinel, and the zero pad.
-__device__ const uint32_t g_cell_f32[2] = {kMissingBits, 0u};
-__device__ const uint64_t g_cell_f64[2] = {kMissingBits64, 0ull};
+// What an uncovered cell copies: the sentinel.
+__device__ const uint32_t g_cell_f32 = kMissingBits;
+__device__ const uint64_t g_cell_f64 = kMissingBits64;
 template <typename T>
-__device__ __forceinline__ const T *no_cell(bool zero) {
+__device__ __forceinline__ const T *no_cell() {
     if constexpr (sizeof(T) == 4)
-        return reinterpret_cast<const T *>(g_cell_f32) + zero;
+        return reinterpret_cast<const T *>(&g_cell_f32);
     else
-        return reinterpret_cast<const T *>(g_cell_f64) + zero;
+        return reinterpret_cast<const T *>(&g_cell_f64);
 }
 
 // The level image: one warp per row (PARTS: per part of `per` cells, where rows
@@ -343,9 +344,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
     const int zs = src_index(z, zn, a.reflect), xs = src_index(x, xn, a.reflect);
     const bool row_in = zs >= 0 && xs >= 0;
     const int first = PARTS ? (int)blockIdx.y * per : 0, end = PARTS ? min(first + per, yn) : yn;  // the warp's cells
-    const T none = (a.reflect || (z >= 0 && z < zn && x >= 0 && x < xn)) ? VT<T>::miss() : T(0);
     if (!row_in) {
-        for (int y = first + lane - R; y < end + R; y += 32) row[y] = none;
+        for (int y = first + lane - R; y < end + R; y += 32) row[y] = T(0);
         return;
     }
     const int nw = nword(yn), nwp = nword(a.dp.yn);
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
     const T *own = in + xz_end[a.row_base + srow - 1];
     const T *tr = a.tw ? tree + t_xz_end[a.trow_base + srow - 1] : nullptr;
     const T *par = a.pw ? in + xz_end[a.prow_base + prow - 1] : nullptr;
-    const T *nowhere = no_cell<T>(!VT<T>::is_miss(none));
+    const T *nowhere = no_cell<T>();
     const unsigned b2 = 2 * (lane & 15), low2 = (1u << b2) - 1u, bit = 1u << lane, low = bit - 1u;
     constexpr int U = 4;  // steps of 64 cells with their loads in flight
     const uint2 zero = make_uint2(0u, 0u);
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
         // the R cells before and after the row
         const int y = lane < R ? -1 - lane : yn + lane - R;
         const int ys = src_index(y, yn, a.reflect);
-        T v = a.reflect ? VT<T>::miss() : T(0);
+        T v = T(0);
         if (ys >= 0) {
             const int j = ys >> 5;
             const unsigned b = 1u << (ys & 31);
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) level_image_kerne
             const uint2 wt = WT ? WT[j] : make_uint2(0u, 0u);
             const uint2 wp = WP ? WP[ys >> 6] : make_uint2(0u, 0u);
             const unsigned pb = 1u << ((ys >> 1) & 31);
-            v = none;
+            v = VT<T>::miss();
             if (w.x & b)
                 v = own[w.y + __popc(w.x & (b - 1u))];
             else if (wt.x & b)
@@ -702,6 +702,18 @@ int image_run(const LD &d, bool whole) {
     const int64_t fit = (int64_t)((uint64_t(1) << 30) / (ImageShape<R, T>(d, 0, 1).plane * sizeof(T))) - halo;
     if (whole || fit >= d.zn) return d.zn;
     return (int)std::min<int64_t>(d.zn, std::max<int64_t>(kTZ, fit / kTZ * kTZ));
+}
+
+// Taps of a particle's (2R + 1)^3 whose reflection leaves the level: as many for
+// every particle of it, so those of its first cell are counted.  used[k]: tap k
+// counts (null: all do).
+uint64_t outside_taps(const LD &d, int R, const bool *used = nullptr) {
+    const int S = 2 * R + 1;
+    uint64_t out = 0;
+    for (int k = 0; k < S * S * S; ++k)
+        out += (!used || used[k]) && (src_index(k / (S * S) - R, d.zn, 1) < 0 ||
+                                      src_index(k / S % S - R, d.xn, 1) < 0 || src_index(k % S - R, d.yn, 1) < 0);
+    return out;
 }
 
 // What a warp takes of `rows` rows of n units: the whole row, or halves of it
@@ -989,6 +1001,7 @@ void filter_apply(const Geom &g, const uint64_t *xz_end, const Geom &tg, const u
     const int L = g.l_max;
     unsigned long long *stale = fb.stale.as<unsigned long long>(1);
     APRB_CUDA(cudaMemsetAsync(stale, 0, sizeof(unsigned long long), s));
+    fb.outside = 0;
     tree_means_all<T>(g, xz_end, tg, t_xz_end, fi, in, tree, s);
     if (!plan) return;
     for (int l = L; l >= g.l_min; --l) {
@@ -996,6 +1009,7 @@ void filter_apply(const Geom &g, const uint64_t *xz_end, const Geom &tg, const u
         const int sn = std::min(plan->nstencils - 1, L - l);
         const int side = plan->sides[sn];
         const ConvLevelArgs a = conv_level_args(g, tg, fi, l, side, plan->reflect);
+        if (plan->reflect) fb.outside += fi.level_count[l] * outside_taps(a.d, side / 2);
         if (side == 3)
             launch_conv_level<1, T>(a, *plan, sn, mode, xz_end, in, t_xz_end, tree, out, rl_in, stale, fb, s);
         else
@@ -1018,6 +1032,7 @@ void filter_gradient_magnitude(const Geom &g, const uint64_t *xz_end, const Geom
     const int L = g.l_max;
     unsigned long long *stale = fb.stale.as<unsigned long long>(1);
     APRB_CUDA(cudaMemsetAsync(stale, 0, sizeof(unsigned long long), s));
+    fb.outside = 0;
     tree_means_all<float>(g, xz_end, tg, t_xz_end, fi, in, tree, s);
     for (int l = L; l >= g.l_min; --l) {
         if (fi.level_count[l] == 0) continue;
@@ -1027,14 +1042,17 @@ void filter_gradient_magnitude(const Geom &g, const uint64_t *xz_end, const Geom
         bool full = false;  // some tap lies off the axes
         for (int d = 0; d < 3; ++d) {
             gw.active[d] = active[d];
+            bool used[27];
             for (int k = 0; k < 27; ++k) {
                 const float w = active[d] ? stencils[d][27 * sn + k] : 0.0f;
                 gw.w[d][k] = w;
+                used[k] = w != 0.0f;
                 if (w == 0.0f) continue;
                 const int id[3] = {k % 3, k / 3 % 3, k / 9};
                 full = full || id[(d + 1) % 3] != 1 || id[(d + 2) % 3] != 1;
                 gw.zuse[k / 9] = 1;
             }
+            fb.outside += fi.level_count[l] * outside_taps(a.d, 1, used);
         }
         // in place, the whole level is read before any of it is written
         const int run = image_run<1, float>(a.d, in == out);
@@ -1058,7 +1076,7 @@ uint64_t filter_stale_count(FilterBuffers &fb, cudaStream_t s) {
     unsigned long long v = 0;
     APRB_CUDA(cudaMemcpyAsync(&v, fb.stale.as<unsigned long long>(1), sizeof(v), cudaMemcpyDeviceToHost, s));
     APRB_CUDA(cudaStreamSynchronize(s));
-    return v;
+    return v + fb.outside;
 }
 
 }  // namespace aprb

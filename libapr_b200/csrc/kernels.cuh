@@ -159,7 +159,8 @@ void launch_tree_fill(const Geom &tg, const DevBuf &flags, const uint64_t *t_xz_
 
 // ---- filter.cu
 struct FilterBuffers {
-    DevBuf dense, stale;
+    DevBuf dense, stale;   // stale: the sentinels that the sums read
+    uint64_t outside = 0;  // taps whose reflection leaves their level, of the last call
 };
 // APRTreeNumerics::fill_tree_mean, or (stencil != null) APRFilter::convolve_pencil
 // whose epilogue is: mode 0 out = conv; mode 1 out = in_u16 / conv (RL ratio);

@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 
 # (z, x, y): words of 32 cells in y, tiles of 16 x 128 cells and 8 planes
 FILTER_SHAPES = [((1, 1, 100), 3), ((1, 40, 65), 6), ((2, 17, 129), 8), ((9, 33, 128), 12), ((8, 16, 66), 6),
-                 ((33, 18, 131), 20), ((17, 50, 257), 20), ((3, 3, 3), 1)]
+                 ((33, 18, 131), 20), ((17, 50, 257), 20), ((3, 3, 3), 1), ((33, 1, 34), 4), ((20, 2, 40), 5),
+                 ((2, 2, 66), 2), ((5, 70, 2), 3)]
 
 
 def built(shape, blobs, image_type=0, seed=11, img=None, **kw):

@@ -1,8 +1,10 @@
-"""The runs of planes that a level's neighbourhood image is made in, checked on
-the CPU: ImageShape and image_run are taken verbatim from
+"""Host rules of a level's neighbourhood image, checked on the CPU: ImageShape,
+image_run, row_part, src_index and outside_taps are taken verbatim from
 libapr_b200/csrc/filter.cu and compiled with g++.  The image of a run, its halo
 planes included, takes at most 1 GiB, or a tile's eight planes and their halo
-where those are more; runs are whole tiles; in place, one run has all planes."""
+where those are more; runs are whole tiles; in place, one run has all planes.
+Parts of a row are whole steps that cover it.  The taps whose reflection leaves a
+level are as many for each of its cells as the count says."""
 import os
 import shutil
 import subprocess
@@ -28,8 +30,38 @@ static long check(int xn, int yn, int zn) {
     return bad;
 }
 
+static long check_outside(int R, int zn, int xn, int yn) {
+    const int S = 2 * R + 1;
+    const LD d{yn, xn, zn};
+    const uint64_t count = outside_taps(d, R);
+    long bad = 0;
+    for (int z = 0; z < zn; ++z)
+        for (int x = 0; x < xn; ++x)
+            for (int y = 0; y < yn; ++y) {
+                uint64_t n = 0;
+                for (int k = 0; k < S * S * S; ++k)
+                    n += src_index(z + k / (S * S) - R, zn, 1) < 0 || src_index(x + k / S % S - R, xn, 1) < 0 ||
+                         src_index(y + k % S - R, yn, 1) < 0;
+                bad += n != count;
+            }
+    return bad;
+}
+
+static long check_part(uint64_t rows, int n, int step, uint64_t warps) {
+    const int per = row_part(rows, n, step, warps);
+    const uint64_t parts = (uint64_t)((n + per - 1) / per);
+    return per % step != 0 || per < step || (rows >= warps && parts != 1) ||
+           (rows * parts < warps && per != step) || parts > 65535;
+}
+
 int main() {
     long bad = 0;
+    for (int zn = 1; zn < 6; ++zn)
+        for (int xn = 1; xn < 6; ++xn)
+            for (int yn = 1; yn < 6; ++yn) bad += check_outside(1, zn, xn, yn) + check_outside(2, zn, xn, yn);
+    for (uint64_t rows : {1, 2, 7, 100, 1000, 4735, 4736, 5919, 5920, 100000})
+        for (int n : {1, 2, 3, 31, 33, 255, 256, 257, 2047, 2048, 2049, 65535})
+            bad += check_part(rows, n, 2, 148 * 8) + check_part(rows, n, 256, 148 * 40);
     for (int side : {1, 3, 100, 1000, 2048, 2900, 3400, 4096, 5800, 8192, 16384, 65535})
         for (int yn : {side, side / 2 + 1})
             for (int zn : {1, 7, 8, 9, 23, 24, 64, 67, 512, 2000, 65535}) {
@@ -52,8 +84,11 @@ def test_image_runs_keep_their_bound(tmp_path):
         return src[a:src.index(end, a) + len(end)]
 
     body = "".join([block("struct LD {", "};\n"), block("template <int R, typename T>\nstruct ImageShape {", "\n};\n"),
-                    block("constexpr int kTX", "\n"), block("template <int R, typename T>\nint image_run(")])
+                    block("constexpr int kTX", "\n"), block("__host__ __device__ __forceinline__ int src_index("),
+                    block("template <int R, typename T>\nint image_run("), block("int row_part("),
+                    block("uint64_t outside_taps(")])
     text = ("#include <algorithm>\n#include <cstdint>\n#include <cstdio>\n#define __host__\n#define __device__\n"
+            "#define __forceinline__ inline\n"
             + body + MAIN)
     path = tmp_path / "image_run.cpp"
     path.write_text(text)
