@@ -39,6 +39,23 @@ def test_filters_at_edges(shape, blobs):
     check_filters(*built(shape, blobs))
 
 
+@pytest.mark.parametrize("weight", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("ks", [3, 5])
+def test_weights_that_are_not_finite_on_a_plane(ks, weight):
+    """A stencil's taps beside a single plane are 0 times their weight: not a number
+    where the weight is not finite, in float and in double."""
+    img, acc, apr = built((1, 40, 65), 6)
+    raw = B.orc_sample(acc, img)
+    st = random_stencil(ks, 5)
+    st[0] = weight
+    for reflect in (True, False):
+        out = A.APRFilter.convolve_pencil(apr, st, raw.astype(np.float32), reflect_boundary=reflect,
+                                          use_stencil_downsample=False, normalize=False)
+        assert np.isnan(out).all()
+    out = A.APRNumerics.richardson_lucy(apr, raw, None, st, 1, use_stencil_downsample=False, dtype=np.float64)
+    assert np.isnan(out).all()
+
+
 def crossed(shape, seed):
     """A volume with a bright ridge across every y that is a multiple of 1024: rows
     stage their words 2048 cells (parents: 1024) at a time."""
