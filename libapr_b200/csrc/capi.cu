@@ -820,6 +820,10 @@ aprb_status aprb_get_apr_from_pyramid_device(aprb_converter *c, const aprb_param
         ARG_CHECK(c && p && pyramid_dev && out, "null argument");
         ARG_CHECK(y_num >= 1 && x_num >= 1 && z_num >= 1 && y_num <= 65535 && x_num <= 65535 && z_num <= 65535,
                   "invalid dimensions");
+        if (c->image_type == APRB_IMAGE_U16 && !c->offset.p) {  // float images have no offset
+            set_error("the converter has filled no tile, so the offset of its working image is not known");
+            throw Error{APRB_ERR_CUDA};
+        }
         cudaStream_t s = (cudaStream_t)stream;
         std::unique_ptr<aprb_apr> a(new aprb_apr());
         init_apr_geometry(a.get(), y_num, x_num, z_num);

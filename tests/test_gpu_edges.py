@@ -231,6 +231,31 @@ def test_block_patches(shape, zb, ghost):
     assert np.array_equal(xe, acc.xz_end) and np.array_equal(yv, acc.y_vec)
 
 
+def test_pyramid_solved_by_a_converter_that_filled_no_tile():
+    """A uint16 APR records the offset of the image it was made from, which only a
+    converter that filled a tile knows: the call is refused.  Float images have none."""
+    import torch
+    from libapr_b200.distributed import TileBackend, tile_count
+    shape, zb, ghost = (40, 70, 33), 8, 4
+    img = volume(shape, 12, 23)
+    slab = torch.from_numpy(img.view(np.int16)).cuda()
+    for image_type, name in ((1, "uint16"), (0, "float")):
+        fill, solve = TileBackend(name, lib_params()), TileBackend(name, lib_params())
+        pyr = fill.pyramid(shape)
+        fill.fill(pyr, shape, zb, ghost, 0, tile_count(shape[0], zb), slab, 0)
+        if image_type == 1:
+            with pytest.raises(RuntimeError, match="offset"):
+                solve.finish(pyr, shape)
+            apr = fill.finish(pyr, shape)
+        else:
+            apr = solve.finish(pyr, shape)
+            assert apr.bspline_offset() == 0
+        e, acc = B.orc_get_apr_by_block(img, oracle_params(), image_type, zb, ghost)
+        assert e == 0
+        lx, xe, yv = apr.linear_access()
+        assert np.array_equal(xe, acc.xz_end) and np.array_equal(yv, acc.y_vec)
+
+
 # rows of 4k + 1 .. 4k + 3 samples of a megavoxel or more: lines padded to a
 # multiple of 8 (float ImageType), every stage compared
 @pytest.mark.parametrize("shape", [(64, 130, 129), (33, 250, 130), (17, 260, 259), (40, 100, 267), (1, 4100, 257)])
