@@ -620,7 +620,13 @@ __global__ void __launch_bounds__(128) iir_strided_rcv_kernel(IT *__restrict__ i
 
 // Threads below which the strided passes leave SMs short of warps: a line is a
 // serial chain, so with few lines the time is the chain's, and lines that share
-// a thread only take latency hiding away.
+// a thread only take latency hiding away.  Against no line and against one at 148
+// * 1024 threads, x and z pass in us: 64 x 512 x 592 uint16 (37,888 lines along x)
+// 108 + 101, 313 + 91 and 108 + 76; 128 x 512 x 592 (75,776) 190 + 191, 349 + 182
+// and 169 + 145; 512 x 512 x 592 (303,104) 919 + 894 either way and 546 + 559, so
+// uint16 would gain from one line per thread further up; float, 158 x 400 x 240
+// 54 + 35, 65 + 40 and 54 + 43, 632 x 400 x 240 173 + 160, 173 + 163 and 170 + 193:
+// there the line is right.
 constexpr uint64_t kFewThreads = 148 * 256;
 
 // The x / z pass over nlines lines of n samples: four or two lines per thread
@@ -1880,7 +1886,10 @@ __global__ void pad_lines_kernel(const uint16_t *__restrict__ src, int yn, int p
 // volumes of a megavoxel and more their lines are padded: the y pass reads a
 // padded copy of the input, and the x / z passes treat the padding as lines of
 // its own (never read by the gradient): 201 x 389 x 517, 1458 -> 1336 us a
-// conversion.  Below that there is nothing to gain.
+// conversion.  The gain grows with the rows: 8 x 128 x 1025 578 -> 525 us, 100 x 200
+// x 201 404 -> 390, 40 x 100 x 261 361 -> 355, none on 33 x 250 x 255 and 64 x 130 x
+// 129 (378 and 328 us against 375 and 324); half a megavoxel and less loses 0 - 3 %
+// (60 x 60 x 133 292 us both, 20 x 100 x 129 281 -> 289), hence the line.
 int work_pitch(int yn, int xn, int zn) {
     const bool pad = yn % 4 != 0 && yn >= 64 && (uint64_t)xn * zn >= 32 && (uint64_t)yn * xn * zn >= (uint64_t(1) << 20);
     return pad ? (yn + 7) & ~7 : yn;
