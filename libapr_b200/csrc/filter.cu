@@ -314,7 +314,7 @@ __device__ __forceinline__ const T *no_cell() {
 // (particle, parent, tree mean) and at which index, so every cell is one load
 // and one store, with no prefill and no y coordinates read.  Rows that no
 // particle of the level is within R of are not written (nothing reads them).
-// Bound by latency and issue slots: 3.8 ms for all levels of the 512 x 2048 x
+// Bound by latency and issue slots: 3.7 ms for all levels of the 512 x 2048 x
 // 2048 APR.  The words of 2048 cells come to shared memory at once, so a step
 // waits for its values only (words read in each step: 4.6 ms; one step ahead in
 // registers: 5.2; a word of 32 cells a step instead of 64 in pairs: 5.6).

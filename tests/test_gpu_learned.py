@@ -98,8 +98,8 @@ def test_trained_proposal_gains_over_the_method_without_it(i):
     plain RL's iterate i + 10 than iterate i itself (measured: 31 - 34 %
     closer) and lowers RL's data-fit objective, so RL keeps it; the same
     network untrained moves the estimate away.  The gain is about three
-    iterations per proposal, against a cost of eight and a half (85 ms per
-    proposal, 10 ms per iteration on 256x1024x1024), so learned RL does not
+    iterations per proposal, against a cost of sixteen (74 ms per proposal,
+    4.65 ms per iteration on 256x1024x1024), so learned RL does not
     reach the 500-iteration FP64 solution sooner than plain RL."""
     import torch
     from libapr_b200 import learned as Lr
