@@ -114,11 +114,11 @@ struct TreeLevelArgs {
 };
 
 // One warp per parent row, or per part of `per` words of one where rows are long
-// and few, a lane per cell of a parent word.  The parent's word
-// gives the node's index, the words of the four child rows each child pair's
-// source and index, so every load of a node's eight children follows from
-// words alone (a row's nodes are neighbours, and so are their children): no
-// y coordinates; two words a step keep sixteen children a lane in flight.
+// and few, a lane per cell of a parent word.  The parent's word gives the node's
+// index, the words of the four child rows each child pair's source and index, so
+// every load of a node's eight children follows from words alone (a row's nodes
+// are neighbours, and so are their children): no y coordinates; two words a step
+// keep sixteen children a lane in flight.
 // Bound by latency: the words come to shared memory 32 at a time, so a step
 // waits for its children only.  512 x 2048 x 2048 APR, all levels: 1.8 ms (words
 // read in each step 3.9, one step ahead in registers 3.2, child rows staged in
@@ -310,10 +310,11 @@ __device__ __forceinline__ const T *no_cell() {
 }
 
 // The level image: one warp per row (PARTS: per part of `per` cells, where rows
-// are long and few), a lane per pair of cells (2j, 2j + 1), which share their parent.  The row words say which source holds a cell
-// (particle, parent, tree mean) and at which index, so every cell is one load
-// and one store, with no prefill and no y coordinates read.  Rows that no
-// particle of the level is within R of are not written (nothing reads them).
+// are long and few), a lane per pair of cells (2j, 2j + 1), which share their
+// parent.  The row words say which source holds a cell (particle, parent, tree
+// mean) and at which index, so every cell is one load and one store, with no
+// prefill and no y coordinates read.  Rows that no particle of the level is within
+// R of are not written (nothing reads them).
 // Bound by latency and issue slots: 3.7 ms for all levels of the 512 x 2048 x
 // 2048 APR.  The words of 2048 cells come to shared memory at once, so a step
 // waits for its values only (words read in each step: 4.6 ms; one step ahead in
@@ -805,8 +806,8 @@ void launch_conv_level(const ConvLevelArgs &a, const ConvPlan &plan, int sn, int
 // weight is zero (2-D Sobel) adds +-0 to a finite sum, which changes the sum
 // only when it is itself zero, and then only its sign, which the square
 // removes; cells of the block that no tap has are not read.
-// Central differences on the 256 x 1024 x 1024 APR (1.4e8 particles): 0.56 ms
-// of 1.41 ms a call, against 1.27 of 2.33 ms for a gather per particle.
+// Central differences on the 256 x 1024 x 1024 APR (1.4e8 particles): 0.52 ms
+// of 1.38 ms a call, against 1.27 of 2.33 ms for a gather per particle.
 struct GradArg {
     float w[3][27];  // weights of the directions in memory order
     int active[3];   // direction enters the magnitude
